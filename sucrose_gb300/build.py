@@ -28,7 +28,7 @@ FLAGS = ["-O3", "-std=c++17", "-lineinfo", "--expt-relaxed-constexpr", "-Xcompil
 
 
 def _deps():
-    return sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + [os.path.join(ROOT, "include", "sucrose_gpu.h")])
+    return sorted(glob.glob(os.path.join(CSRC, "*.cuh")) + glob.glob(os.path.join(CSRC, "*.h")) + [os.path.join(ROOT, "include", "sucrose_gpu.h")])
 
 
 def _needs(out, srcs):

@@ -22,6 +22,7 @@
 
 #include <cooperative_groups.h>
 
+#include "cell_axis.h"
 #include "f32x2.cuh"
 #include "sg_internal.cuh"
 #include "step_epi.cuh"
@@ -670,17 +671,7 @@ struct CoopBuild {
     int* tmp;   // gridDim.x block totals of the scans
 };
 
-// Cell of a position and the position's image in the box, consistent with
-// each other: whole boxes are taken off both (in FP64 when there are any, so
-// that the image is the position to half an ulp of the box).
-__device__ __forceinline__ int cell_axis(float& x, int nc, float L, float iL, double Ld) {
-    const int c = (int)floorf((x + 0.5f * L) * (nc * iL));
-    if (c >= 0 && c < nc) return c;
-    const int k = c >= 0 ? c / nc : -((nc - 1 - c) / nc);
-    x = (float)((double)x - (double)k * Ld);
-    return c - k * nc;
-}
-
+// Cell of a position and the position's image in the box (cell_axis.h).
 __device__ __forceinline__ int cell_and_image(float4& p, const ListGeom& g) {
     const int cx = cell_axis(p.x, g.nc[0], g.box.x, g.inv_box.x, g.bx);
     const int cy = cell_axis(p.y, g.nc[1], g.box.y, g.inv_box.y, g.by);
