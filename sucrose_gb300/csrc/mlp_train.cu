@@ -419,13 +419,14 @@ int sg_mlp_features(sg_ctx* ctx, void* x_bf16, float* y, int64_t capacity, int64
     const float3 box = make_float3((float)ctx->box[0], (float)ctx->box[1], (float)ctx->box[2]);
     const float3 ib = make_float3((float)(1.0 / ctx->box[0]), (float)(1.0 / ctx->box[1]), (float)(1.0 / ctx->box[2]));
     const long long n = std::min<long long>(k, capacity);
-    if (n > 0)
+    if (n > 0) {
         if (int rc = sg_need_half_list(ctx, true)) return rc;
         k_features<<<(int)((n + 255) / 256), 256, 0, ctx->stream>>>(ctx->nl.pair_i, ctx->nl.pair_j,
                                                                     ctx->nl.dev_flags + 2, ctx->pos, ctx->quat,
                                                                     ctx->shape, ctx->ecp_lambda, box, ib,
                                                                     ctx->periodic, capacity,
                                                                     (__nv_bfloat16*)x_bf16, y);
+    }
     SG_LAUNCH_CHECK(ctx, "k_features");
     SG_CUDA(ctx, cudaStreamSynchronize(ctx->stream));
     *count = n;
