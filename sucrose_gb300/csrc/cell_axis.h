@@ -10,15 +10,16 @@
 #endif
 
 // The cell in [0, nc) of any x, the non-finite ones among them, and x's image
-// in the box, consistent with each other: whole boxes are taken off both (in
-// FP64 when there are any, so that the image is the position to half an ulp of
-// the box). The cell count never leaves floating point before it is known to
-// fit: a coordinate of 2^31 cell widths and more has no int, and the build
-// indexes memory with what comes out.
+// in the box. Outside the box the image comes first, in FP64, and the cell is the
+// image's: an FP32 cell of the coordinate itself is off by 1e-7 of its distance,
+// which some tens of boxes out passes what the row search allows for when it
+// cuts the cells to the reach of its rows. The cell count never leaves floating
+// point before it is known to fit: a coordinate of 2^31 cell widths and more has no
+// int, and the build indexes memory with what comes out.
 SG_CELL_FN int cell_axis(float& x, int nc, float L, float iL, double Ld) {
-    const float f = floorf((x + 0.5f * L) * (nc * iL));
+    float f = floorf((x + 0.5f * L) * (nc * iL));
     if (f >= 0.f && f < (float)nc) return (int)f;
-    const double k = floor((double)f / nc), m = (double)f - k * nc;
-    x = (float)((double)x - k * Ld);
-    return m > 0.0 ? (m < nc ? (int)m : nc - 1) : 0;   // past 2^53 cells, m is rounded; a NaN: cell 0
+    x = (float)((double)x - floor((double)x / Ld + 0.5) * Ld);
+    f = floorf((x + 0.5f * L) * (nc * iL));
+    return f > 0.f ? (f < (float)nc ? (int)f : nc - 1) : 0;   // an image on a face; not finite, or past FP64
 }
