@@ -5,7 +5,7 @@
 // so that a formula is written once for both widths.
 #pragma once
 
-#include "sg_internal.cuh"
+#include "dfloat.cuh"
 
 struct f2 {
     unsigned long long v;
@@ -97,3 +97,25 @@ SG_DEV mask2 not_above_w(f2 a, f2 b) {
     f2_split(b, bx, by);
     return {ax <= bx, ay <= by};
 }
+
+// A sum of FP32 terms that loses no rounding error: two-sum's error of every
+// addition goes into lo, so that sum and lo together hold about 48 bits whatever
+// the terms' sizes and signs (Kahan's form, four instructions instead of seven,
+// is exact only while the sum is the larger operand: 3e-9 of the terms'
+// magnitudes on terms of both signs).
+struct F2Sum {
+    f2 hi, lo;
+    SG_DEV void add(f2 v) {
+        const f2 s = hi + v, b = s - hi;
+        lo = lo + ((hi - (s - b)) + (v - b));
+        hi = s;
+    }
+    // both halves, as hi + lo
+    SG_DEV dfl total() const {
+        float x, y, xl, yl;
+        f2_split(hi, x, y);
+        f2_split(lo, xl, yl);
+        const dfl d = df_two_sum(x, y);
+        return {d.hi, d.lo + (xl + yl)};
+    }
+};

@@ -385,14 +385,14 @@ struct GbWarp {
     int lane;
     int nm = 0, hm = 0, nn = 0, hn = 0;   // waiting pairs and ring heads
     unsigned ranged = 0, precise = 0;
-    f2 pe, pe_c, vir, vir_c;              // Kahan sums (see RowSums)
+    F2Sum pe, vir;
     EnergySums es;                        // of the near-contact class
     int row = -1;                         // the row whose sums are held
     float3 f, t;
 
     SG_DEV GbWarp(const PairLaunch& l, const PotGB<KIND>& p, GbQueue* m, GbQueue* n, GbAxes* a)
         : L(l), pot(p), main(m), near(n), axes(a), lane(threadIdx.x & 31) {
-        pe = pe_c = vir = vir_c = all_w<f2>(0.f);
+        pe = vir = F2Sum{all_w<f2>(0.f), all_w<f2>(0.f)};
         f = t = make_float3(0.f, 0.f, 0.f);
         box = pot.b.box;
         inv_box = pot.b.periodic ? pot.b.inv_box : f;
@@ -524,13 +524,8 @@ struct GbWarp {
         if (L.stats) ranged += __popc(__ballot_sync(full, act.lo)) + __popc(__ballot_sync(full, act.hi));
         {
             const f2 zero = all_w<f2>(0.f);
-            f2 y = select_w(act, o.pe, zero) - pe_c, s = pe + y;
-            pe_c = (s - pe) - y;
-            pe = s;
-            y = select_w(act, o.vir, zero) - vir_c;
-            s = vir + y;
-            vir_c = (s - vir) - y;
-            vir = s;
+            pe.add(select_w(act, o.pe, zero));
+            vir.add(select_w(act, o.vir, zero));
         }
         float3 f0, f1, t0, t1, s0, s1;
         f2_split(o.fx, f0.x, f1.x); f2_split(o.fy, f0.y, f1.y); f2_split(o.fz, f0.z, f1.z);
@@ -692,16 +687,13 @@ __global__ void __launch_bounds__(SG_PAIR_MAX_BLOCK, SG_GB_BLOCKS) k_pair_gb(Pai
         if (g.precise) atomicAdd(&L.stats[3], (unsigned long long)g.precise);
     }
     float e[2], elo[2];
-    auto total = [](f2 s, f2 c, float x, float x_lo, float& hi, float& low) {
-        float a, b, ca, cb;
-        f2_split(s, a, b);
-        f2_split(c, ca, cb);
-        const dfl d = df_two_sum(a, b), t = df_two_sum(d.hi, x);
+    auto total = [](const F2Sum& s, float x, float x_lo, float& hi, float& low) {
+        const dfl d = s.total(), t = df_two_sum(d.hi, x);
         hi = t.hi;
-        low = t.lo + d.lo + x_lo - (ca + cb);
+        low = t.lo + d.lo + x_lo;
     };
-    total(g.pe, g.pe_c, g.es.pe, g.es.pe_lo, e[0], elo[0]);
-    total(g.vir, g.vir_c, g.es.vir, g.es.vir_lo, e[1], elo[1]);
+    total(g.pe, g.es.pe, g.es.pe_lo, e[0], elo[0]);
+    total(g.vir, g.es.vir, g.es.vir_lo, e[1], elo[1]);
     pair_sums_finish(e, elo, L.partials, L.done, L.acc, L.acc_total);
 }
 
