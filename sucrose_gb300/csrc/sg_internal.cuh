@@ -11,6 +11,7 @@
 #include <vector>
 
 #include "../../include/sucrose_gpu.h"
+#include "graph_steps.h"
 
 #define SG_DEV __device__ __forceinline__
 
@@ -266,11 +267,10 @@ struct sg_ctx {
     // final half stored (nothing can change the state between those launches)
     cudaGraphExec_t graph_exec_cont = nullptr;
     int step_sums_from_acc = 0;      // set while enqueuing that step
-    // several steps in one graph (sg_step): graph_multi_steps copies of step_graph
+    // several steps in one graph (sg_step): graph_steps.steps copies of step_graph
     cudaGraph_t step_graph = nullptr;
     cudaGraphExec_t graph_multi = nullptr;
-    int graph_multi_steps = 0;
-    int step_calls = 0;              // sg_step calls since the step was captured
+    GraphSteps graph_steps;
     // host calls that write the particle state bump state_version; sg_step
     // records it after its launches, so that the first launch of the next
     // call may take the stored sums only when nothing was written in between

@@ -241,35 +241,17 @@ void drop_graphs(sg_ctx* ctx) {
     ctx->graph_exec = nullptr;
     ctx->graph_exec_cont = nullptr;
     ctx->graph_multi = nullptr;
-    ctx->graph_multi_steps = 0;
+    ctx->graph_steps = GraphSteps();
     ctx->step_graph = nullptr;
-    ctx->step_calls = 0;
 }
 
-// Steps in one graph: copies of the captured step, one after the other. Between
-// two graph launches the stream idles for 3.5 to 5 us; inside a graph kernels
-// follow each other in 0.1 to 0.3. 30 steps of 2 916 LJ particles take 726 us in
-// graphs of one step and 631 in graphs of 15, 20 ECP steps of 65 536 particles
-// 1229 and 1132, 10 chain steps of 96 000 beads 928 and 911. The graph holds a
-// whole fraction of the steps that the caller asks for at a time, at most
-// SG_GRAPH_STEPS: past that a gap is less than 0.3 us a step. Putting it
-// together costs the host some 7 us a node (430 us for 15 steps of four
-// kernels), more than a few steps gain, so the second call with the captured
-// step makes it, or a first one of many steps. It is replaced only by one four
-// times as long, so that calls of changing lengths do not make it over and
-// over. Replica steps hold a conditional node, which a child graph may not, and
+// Steps in one graph (graph_steps.h): copies of the captured step, one after the
+// other. Replica steps hold a conditional node, which a child graph may not, and
 // take milliseconds.
-#define SG_GRAPH_STEPS 16
-int multi_steps(const sg_ctx* ctx, int nsteps) {
-    if (!ctx->step_graph || nsteps < 2) return 0;
-    if (ctx->step_calls < 2 && nsteps < 4 * SG_GRAPH_STEPS) return 0;
-    return nsteps / ((nsteps + SG_GRAPH_STEPS - 1) / SG_GRAPH_STEPS);
-}
-
 int make_multi(sg_ctx* ctx, int steps) {
     if (ctx->graph_multi) cudaGraphExecDestroy(ctx->graph_multi);
     ctx->graph_multi = nullptr;
-    ctx->graph_multi_steps = 0;
+    ctx->graph_steps.made(0);
     cudaGraph_t graph = nullptr;
     cudaGraphNode_t prev = nullptr, node = nullptr;
     SG_CUDA(ctx, cudaGraphCreate(&graph, 0));
@@ -284,7 +266,7 @@ int make_multi(sg_ctx* ctx, int steps) {
         ctx->graph_multi = nullptr;
         return sg_cuda_check(ctx, e, "graph of several steps");
     }
-    ctx->graph_multi_steps = steps;
+    ctx->graph_steps.made(steps);
     return SG_OK;
 }
 
@@ -344,15 +326,15 @@ int sg_step(sg_ctx* ctx, int32_t nsteps) {
     // a launch after a step of this call, or after one of an earlier call
     // with no state written since, takes the stored sums; otherwise the step
     // recomputes them
-    if (nsteps > 0 && ctx->step_calls < 2) ctx->step_calls++;
-    const int want = multi_steps(ctx, nsteps - done);
-    if (want > 1 && (!ctx->graph_multi || want >= 4 * ctx->graph_multi_steps))
+    if (const int want = ctx->step_graph ? ctx->graph_steps.wanted(nsteps - done, ctx->graph_kernels) : 0)
         if (int rc = make_multi(ctx, want)) return rc;
+    const int multi = ctx->graph_steps.steps;
     for (int s = done; s < nsteps;) {
         const bool cont = s > 0 || clean;
-        if (ctx->graph_multi && nsteps - s >= ctx->graph_multi_steps && (cont || !ctx->graph_exec_cont)) {
+        ctx->graph_steps.gaps++;
+        if (ctx->graph_multi && nsteps - s >= multi && (cont || !ctx->graph_exec_cont)) {
             SG_CUDA(ctx, cudaGraphLaunch(ctx->graph_multi, ctx->stream));
-            s += ctx->graph_multi_steps;
+            s += multi;
             continue;
         }
         SG_CUDA(ctx, cudaGraphLaunch(cont && ctx->graph_exec_cont ? ctx->graph_exec_cont : ctx->graph_exec, ctx->stream));
