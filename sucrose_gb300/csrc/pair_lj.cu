@@ -50,7 +50,7 @@ int sg_launch_pair_simple(sg_ctx* ctx, const sg_pair_params* p) {
 // system with rows. Each neighbour's position is fetched once for both: WCA and
 // Coulomb on 131 072 charged spheres 65 us together, 46 and 63 us apart.
 bool sg_pair_sets_fuse(const sg_ctx* ctx, const sg_pair_params* a, const sg_pair_params* b) {
-    return rows_apply(ctx) && a->kind <= SG_WCA && b->kind >= SG_MORSE && b->kind <= SG_COULOMB;
+    return rows_apply(ctx) && a->kind >= SG_LJ && a->kind <= SG_WCA && b->kind >= SG_MORSE && b->kind <= SG_COULOMB;
 }
 
 int sg_launch_pair_both(sg_ctx* ctx, const sg_pair_params* a, const sg_pair_params* b) {
