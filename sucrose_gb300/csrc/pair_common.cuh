@@ -165,8 +165,8 @@ struct EnergySums {
 
 // One pair per lane, evaluated and scattered (all 32 lanes call it).
 // i, j: the pair's particles (loaded by the caller; ignored when !valid).
-// COUNT: 0 nothing, 1 listed and in-range pairs, 2 in-range pairs only.
-template <class Pot, int COUNT>
+// COUNT: listed and in-range pairs are counted here.
+template <class Pot, bool COUNT>
 SG_DEV void pair_process(const PairLaunch& L, const Pot& pot, int t, int i, int j, bool valid, EnergySums& es,
                          unsigned long long* sh_stats) {
     const int lane = threadIdx.x & 31;
@@ -187,7 +187,7 @@ SG_DEV void pair_process(const PairLaunch& L, const Pot& pot, int t, int i, int 
         // stats[0] listed pairs, stats[1] pairs inside the range
         const unsigned va = __ballot_sync(0xffffffffu, valid), ac = __ballot_sync(0xffffffffu, o.act != 0);
         if (lane == 0) {
-            if (COUNT == 1) atomicAdd(&sh_stats[0], (unsigned long long)__popc(va));
+            atomicAdd(&sh_stats[0], (unsigned long long)__popc(va));
             if (ac) atomicAdd(&sh_stats[1], (unsigned long long)__popc(ac));
         }
     }
@@ -205,9 +205,8 @@ SG_DEV void pair_process(const PairLaunch& L, const Pot& pot, int t, int i, int 
 // idles on an out-of-range pair. Slots: storage index, i, j; 64 a warp.
 template <class Pot>
 struct PairQueues {
-    static constexpr bool kExact = ExactFilter<Pot>::value;
+    static_assert(!Pot::kCountActive || ExactFilter<Pot>::value, "in_range counts for eval");
     static constexpr int kWords = 64 * 3;   // shared words per warp
-    static constexpr int kCnt = (Pot::kCountActive && !kExact) ? 2 : 0;
     int* q;   // this warp's queue: t at +0, i at +64, j at +128
     int qn;
     int lane;
@@ -241,7 +240,7 @@ struct PairQueues {
         }
         __syncwarp();
         qn -= n;
-        pair_process<Pot, kCnt>(L, pot, tq, iq, jq, ok, es, sh_stats);
+        pair_process<Pot, false>(L, pot, tq, iq, jq, ok, es, sh_stats);
     }
     // one listed pair per lane: range test, counters, queue, evaluate full batches
     SG_DEV void feed(const PairLaunch& L, const Pot& pot, int t, int i, int j, bool valid, EnergySums& es,
@@ -250,7 +249,7 @@ struct PairQueues {
         const unsigned vm = __ballot_sync(0xffffffffu, valid), km = __ballot_sync(0xffffffffu, in);
         if (Pot::kCountActive && lane == 0) {
             atomicAdd(&sh_stats[0], (unsigned long long)__popc(vm));
-            if (kExact && km) atomicAdd(&sh_stats[1], (unsigned long long)__popc(km));
+            if (km) atomicAdd(&sh_stats[1], (unsigned long long)__popc(km));
         }
         if constexpr (Pot::kStats) {
             // solver statistics (ECP): a pair turned away counts as listed with
@@ -271,10 +270,15 @@ struct PairQueues {
     }
 };
 
+template <class Pot, bool FILTER>
+constexpr int pair_min_blocks() {
+    if constexpr (FILTER) return Pot::kMinBlocksFiltered;
+    else return Pot::kMinBlocks;
+}
+
 // FILTER: the range test and per-warp queues of PairQueues.
 template <class Pot, bool FILTER>
-__global__ void __launch_bounds__(SG_PAIR_MAX_BLOCK, FILTER ? Pot::kMinBlocksFiltered : Pot::kMinBlocks)
-    k_pair(PairLaunch L, Pot pot) {
+__global__ void __launch_bounds__(SG_PAIR_MAX_BLOCK, (pair_min_blocks<Pot, FILTER>())) k_pair(PairLaunch L, Pot pot) {
     using Q = PairQueues<Pot>;
     __shared__ unsigned long long sh_stats[SG_NSTATS];
     __shared__ int sh_queue[FILTER ? (SG_PAIR_MAX_BLOCK / 32) * Q::kWords : 1];
@@ -302,7 +306,7 @@ __global__ void __launch_bounds__(SG_PAIR_MAX_BLOCK, FILTER ? Pot::kMinBlocksFil
         const bool valid = vn;
         if (base + stride < np) pair_fetch(L, base + stride, lane, np, b0, tn, in_, jn, vn);   // next indices in flight
         if constexpr (!FILTER)
-            pair_process<Pot, Pot::kCountActive ? 1 : 0>(L, pot, t, i, j, valid, es, sh_stats);
+            pair_process<Pot, Pot::kCountActive>(L, pot, t, i, j, valid, es, sh_stats);
         else
             q.feed(L, pot, t, i, j, valid, es, sh_stats);
     }
@@ -414,7 +418,7 @@ __global__ void __launch_bounds__(SG_PAIR_MAX_BLOCK, BLOCKS) k_pair_tested(PairL
             const bool ok = 32 * b + lane < n;
             const int s = ok ? 32 * b + lane : 0;
             if (lane == 0) b = atomicAdd(&sh_next, 1);
-            pair_process<Pot, 0>(L, pot, qt[s], qi[s], qj[s], ok, es, sh_stats);
+            pair_process<Pot, false>(L, pot, qt[s], qi[s], qj[s], ok, es, sh_stats);
             b = __shfl_sync(full, b, 0);
         }
         if (last) break;
@@ -454,7 +458,7 @@ PairTune sg_pair_tune_for(sg_ctx* ctx, int kind, bool filterable);
 
 template <class Pot, bool FILTER>
 int launch_pair_v(sg_ctx* ctx, PairLaunch L, Pot pot, int block) {
-    pot.prefiltered = (FILTER && ExactFilter<Pot>::value) ? 1 : 0;
+    if constexpr (Pot::kFilterable) pot.prefiltered = (FILTER && ExactFilter<Pot>::value) ? 1 : 0;
     const void* fn = (const void*)k_pair<Pot, FILTER>;
     int grid = sg_grid_for(ctx, fn, block, 0);
     int64_t max_useful = (ctx->nl.pair_capacity + block - 1) / block;

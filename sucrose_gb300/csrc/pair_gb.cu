@@ -244,15 +244,12 @@ struct PotGB {
     static constexpr bool kWeld = (KIND == SG_GBW || KIND == SG_GBWC);
     static constexpr bool kFilterable = false;   // the filtered launch is k_pair_gb
     static constexpr int kMinBlocks = 1;
-    static constexpr int kMinBlocksFiltered = 1;
-    const float4* __restrict__ pos;
     const float4* __restrict__ prep;   // rec: 2 per particle
     const float4* __restrict__ aux;    // 1 per particle
     const float4* __restrict__ lo;     // 1 per particle: low parts of u and chi
     BoxF b;
     float cutoff, wf, chirality;
     int mu, nu;
-    int prefiltered;   // eval only sees pairs that passed an exact range test
 
     // A superset of eval's range test (r against the orientation-dependent
     // contact distance sigma of I's shape plus the cut-off), without its
@@ -279,10 +276,6 @@ struct PotGB {
     }
     SG_DEV float reach_shift() const {
         return (KIND == SG_GBR) ? 0.f : kWeld ? (cutoff + wf - 1.f) : (cutoff - 1.f);
-    }
-    SG_DEV bool in_range(int i, int j) const {
-        float3 r;
-        return in_range_r(i, j, r) != 0;
     }
 
     // unfiltered launch: the range test's class picks the evaluation, as the
@@ -330,7 +323,7 @@ struct PotGB {
         }
         GbOut<float> w;
         const bool active = gb_eval<KIND, PRECISE>(p, c, cutoff, wf, chirality, mu, nu, w);
-        if (!(active || prefiltered)) return;
+        if (!active) return;
         o.act = 1;
         o.pe = w.pe;
         o.vir = w.vir;
@@ -361,9 +354,7 @@ struct PotGB {
 // cost twice the wavefronts (99 us), in registers more of those than it hid (103).
 #define SG_GB_SLOTS 128   // ring of 64 to 127 waiting pairs: a chunk adds 64 at most
 #define SG_GB_ROWS 6      // more rows than this in a batch: segmented sums
-#ifndef SG_GB_BLOCKS
 #define SG_GB_BLOCKS 2
-#endif
 
 struct GbQueue {   // one warp's waiting pairs of one class: r_ij
     int i[SG_GB_SLOTS], j[SG_GB_SLOTS];
@@ -717,8 +708,6 @@ int launch_gb_pairs(sg_ctx* ctx, const PotGB<KIND>& pot, int block) {
 template <int KIND>
 int launch_gb(sg_ctx* ctx, const sg_pair_params* p, float4* prep, int mu, int nu) {
     PotGB<KIND> pot;
-    pot.prefiltered = 0;
-    pot.pos = ctx->pos;
     pot.prep = prep;
     pot.aux = prep + 2 * (size_t)ctx->n;
     pot.lo = prep + 3 * (size_t)ctx->n;
