@@ -901,6 +901,8 @@ def run_constrained(a):
     ta = stages["constraints_a"] * 1e-3
     bytes_a = nc * (2 * 16 * 2 + 2 * 16 * 2 + 2 * 16 + 12)
     e2e_value, h2d, d2h = e2e_rate(g, torch, max(10, a.steps // 4), nc)
+    # molecules of single bonds, or of three atoms and more (which have an atom in two bonds)
+    kname = "k_rattle_wave" if np.bincount(np.concatenate([bbi, bbj])).max() > 1 else "k_rattle_a"
     if rank == 0:
         line = {
             "metric": w["metric"],
@@ -917,7 +919,7 @@ def run_constrained(a):
             "pair_evals_per_s": npairs * a.steps * world / t_dev,
             "e2e": {"value": e2e_value, "unit": "constraint-solves/s", "h2d_bytes_per_step": h2d, "d2h_bytes_per_step": d2h},
             "gpu_launches": int(kernels_per_step * a.steps),
-            "roofline": {"bound": "hbm", "kernel": "k_rattle_a", "achieved": bytes_a / ta / 1e9 if ta > 0 else None,
+            "roofline": {"bound": "hbm", "kernel": kname, "achieved": bytes_a / ta / 1e9 if ta > 0 else None,
                          "peak": hbm, "unit": "GB/s", "frac": (bytes_a / ta / 1e9 / hbm) if (hbm and ta > 0) else None,
                          "bytes_per_launch": "124 per constraint (one correction)", "traffic": None,
                          "peak_source": "MEASURED_PEAKS.json hbm_gbs (copy bandwidth)"},
@@ -1242,6 +1244,9 @@ def replicas_line(a, rank=0, world=1, local=0, dist=None, steps=None):
         fam[name] = {"listed_pairs": int(st.pairs), "in_range": int(st.solver_evals), "force_kernel_ms": 1e3 * tk,
                      "tflops": fl / tk / 1e12}
     top = max(fam, key=lambda k: fam[k]["force_kernel_ms"])
+    # by the launch that the autotuner picked
+    kname = {("GB", 0): "k_pair<PotGB>", ("GB", 1): "k_pair_gb", ("LJ", 0): "k_pair_spans<PotLJ>",
+             ("LJ", 1): "k_pair<PotLJ, filtered>"}[top, tunes[top]["filter"]] + " (replica family range)"
 
     # e2e through the C ABI: FP64 host state in and out every step
     n = g.n
@@ -1321,7 +1326,7 @@ def replicas_line(a, rank=0, world=1, local=0, dist=None, steps=None):
             "e2e": {"value": npairs * e_steps / t_e2e, "unit": "pair-evals/s", "h2d_bytes_per_step": 13 * 8 * n,
                     "d2h_bytes_per_step": 13 * 8 * n + 32},
             "gpu_launches": int(kernels_per_step * steps),
-            "roofline": {"bound": "fp32", "kernel": "k_pair_gb" if top == "GB" else f"k_pair<Pot{top}> (replica family range)",
+            "roofline": {"bound": "fp32", "kernel": kname,
                          "achieved": fam[top]["tflops"], "peak": peak32, "unit": "TFLOP/s",
                          "frac": fam[top]["tflops"] / peak32,
                          "peak_source": "measured FMA throughput (sg_peak_fma) on this GPU", "traffic": None},
