@@ -1514,7 +1514,10 @@ own filter (for example ncu -k regex:k_pair -c 2). Cases:
   mlp_train one MLP training step on 65 536 samples
   ecp_step  captured Nose-Hoover steps of the ECP system (list build as
             flag-gated kernels, so that a profiler sees every kernel)
-  replicas  captured steps of --nrep replicas (LJ + GB), same flag"""
+  charged   captured steps of the charged spheres (WCA and Coulomb in one pass)
+  polymer   captured steps of the bead chains (RATTLE, bends, dihedrals, WCA)
+  replicas  captured steps of --nrep replicas (LJ + GB), same flag
+--rep-equil steps come first, untimed, in the last three."""
 
 
 def profile_case(a):
@@ -1539,6 +1542,27 @@ def profile_case(a):
         g.upload(r=r, v=configs.velocities_to_temperature(len(r), 0.722, 15))
         g.init_nlist(0.3, 2.5, trigger_mode=1)
         p = g.params(capi.LJ, cutoff=2.5)
+    elif case == "charged":
+        w = CHARGED
+        r, q, box, v, charge = charged_state(w["seed"])
+        g = GpuSystem(len(r), box)
+        g.upload(r=r, q=q, v=v)
+        g.set_charges(charge)
+        g.init_nlist(w["skin"], w["cutoff"], trigger_mode=1)
+        g.configure_step_pairs(charged_params(g), integrator=capi.INT_LANGEVIN, dt=w["dt"], target_temp=w["T"],
+                               damping=w["damping"])
+    elif case == "polymer":
+        w = MOLECULAR[case]
+        r, box, bbi, bbj, ln, terms = molecular_state(case, w["seed"])
+        g = GpuSystem(len(r), box)
+        g.upload(r=r, v=configs.velocities_to_temperature(len(r), w["T"], w["seed"]))
+        g.set_constraints(bbi, bbj, ln)
+        for kind, atoms, coeff, angle in terms:
+            g.bonded_set(kind, atoms, coeff, angle)
+        g.init_nlist(w["skin"], w["sigma"], trigger_mode=1)
+        g.configure_step(g.params(capi.WCA, sigma=w["sigma"], cutoff=w["sigma"]), integrator=capi.INT_LANGEVIN,
+                         dt=w["dt"], target_temp=w["T"], damping=w["damping"],
+                         flags=capi.STEP_CONSTRAINTS | capi.STEP_BONDED)
     elif case != "replicas":
         raise SystemExit("unknown case " + case + "\n" + PROFILE_CASES)
     reps = a.reps
@@ -1580,6 +1604,9 @@ def profile_case(a):
         g.configure_step(p, integrator=capi.INT_NH, dt=0.001, target_temp=1.2, rotations=1, rot_chain=1,
                          flags=capi.STEP_FLAT)
         g.step(1 + reps)
+    elif case in ("charged", "polymer"):
+        for _ in range(a.rep_equil + 1 + reps):
+            g.step(1)
     elif case == "mlp_train":
         from sucrose_gb300 import mlp
 

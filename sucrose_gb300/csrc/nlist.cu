@@ -33,9 +33,16 @@ namespace {
 
 // Up to this many particles the full rows list particles, and the row driver
 // reads their positions where they are (half a megabyte, most of it in L1 before
-// long); with more it copies them into cell order first, a launch of 1.4 us and
-// up. LJ calls with and without the copy: 2 916 particles 9.4 and 7.8 us, 20 000
-// 15.2 and 13.8.
+// long); with more it copies them into cell order first, a launch of 1.2 us and
+// up. What the copy gains grows with the rows' length, for particles in random order
+// (any fluid after a while); on rows of a hundred or so, and for particles in
+// spatial order, it costs 1 to 7 % at every size. Pair stage of a captured step, us,
+// with / without the copy, random order: LJ at cut-off 4 (270 a row) 16 384
+// particles 24.1 / 23.2, 27 436 32.3 / 32.3, 131 072 123 / 125, a million 883 / 937;
+// at 6 (900 a row) 131 072 329 / 346, 500 000 1207 / 1351; dipoles 16 384 49.4 /
+// 51.7, 37 044 78.6 / 86.8, 500 000 872 / 1024; LJ at 2.5 (77 a row) 2 916 9.7 /
+// 8.9, 37 044 18.1 / 16.0, a million 250 / 249; charged spheres (115 a row) 131 072
+// 73.9 / 70.9.
 #define SG_ROWS_DIRECT 32768
 
 constexpr int SCAN_BLOCK = 1024;
