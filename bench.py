@@ -190,8 +190,9 @@ NCU_TRAFFIC = {
            "source": "profiles/k_pair_ecp_newton_N65536.md: ncu, 0.46 M listed pairs"},
     "GB": {"bytes": 46.35e6, "pairs": 5.39e6,
            "source": "profiles/k_pair_gb_filtered_N32768.md: ncu, 5.39 M listed pairs"},
-    "COULOMB": {"bytes": 90.24e6, "pairs": 7.99e6,
-                "source": "profiles/k_pair_coulomb_charged_N131072.md: ncu, 7.99 M listed pairs"},
+    "COULOMB": {"bytes": 92.53e6, "pairs": 8.55e6,
+                "source": "profiles/k_pair_coulomb_charged_N131072.md: ncu, 8.55 M listed pairs, WCA in the "
+                          "same pass (rows and positions are read once)"},
 }
 
 
